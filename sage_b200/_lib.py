@@ -1,13 +1,20 @@
-"""ctypes binding of libsage_b200.so (the C ABI declared in include/sage_b200.h).
+"""ctypes binding of libsage_b200.so (the C ABI declared in include/sage_b200.h), and the C++ side of the
+torch operators (`_native.so`).
 
-There is no fallback: if the library is missing or a call fails, an exception is raised.
+Neither is touched at import: `load` brings in both the first time one of them is needed, so a tree may be built
+after the package was imported, and a process that only builds maps no compiled code of this package.
+There is no fallback: if one is missing or a call fails, an exception is raised.
 """
 
 from __future__ import annotations
 
 import ctypes
+import importlib
 import os
 import pathlib
+import threading
+
+import torch
 
 PACKAGE = pathlib.Path(__file__).resolve().parent
 # SAGEB200_LIBRARY selects another build of the same library (the profiling build that
@@ -17,25 +24,11 @@ LIBRARY = pathlib.Path(os.environ.get("SAGEB200_LIBRARY", PACKAGE / "libsage_b20
 OK = 0
 MAX_GROUPED = 16
 
-# The torch operators' C++ side; None only in a tree that has not been built, where `load` raises.
-try:
-    import torch  # noqa: F401  (its libraries have to be in the process first)
-
-    from . import _native as native
-except ImportError:
-    native = None
-
 NATIVE_SYMBOLS = ("sageb200_status_string", "sageb200_workspace_bytes", "sageb200_linear",
                   "sageb200_sph_workspace_bytes", "sageb200_sph_linear_scratch",
                   "sageb200_linear_takes_type", "sageb200_linear_typed",
                   "sageb200_dequant", "sageb200_pack_logits", "sageb200_codebook_logits", "sageb200_invert_permutation")
 
-
-def native_module():
-    """The C++ side, or the error that says how to build it."""
-    if native is None:
-        raise RuntimeError("sage_b200/_native.so is missing: build it with `python -m sage_b200.build`")
-    return native
 
 # every symbol include/sage_b200.h declares
 EXPORTED = (
@@ -213,18 +206,50 @@ class Problem(ctypes.Structure):
 
 
 _handle: ctypes.CDLL | None = None
+_native = None
+_load_lock = threading.RLock()
+
+
+def native_module():
+    """The C++ side of the operators."""
+    if _native is None:
+        load()
+    return _native
 
 
 def load() -> ctypes.CDLL:
-    """Load the shared library once; raise if it has not been built."""
-    global _handle
+    """Load the shared library and the operators' C++ side once; raise if they have not been built."""
+    global _handle, _native
     if _handle is not None:
         return _handle
-    if not LIBRARY.exists():
-        raise RuntimeError(
-            f"{LIBRARY} is missing: build it with `python -m sage_b200.build` "
-            "(sage_b200 has no CPU or PyTorch fallback)"
-        )
+    with _load_lock:
+        if _handle is None:
+            if not LIBRARY.exists():
+                raise RuntimeError(
+                    f"{LIBRARY} is missing: build it with `python -m sage_b200.build` "
+                    "(sage_b200 has no CPU or PyTorch fallback)"
+                )
+            lib, module = _bind_library(), _import_native()
+            module.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in NATIVE_SYMBOLS})
+            while _unregistered:
+                module.register_kernels(*_unregistered.pop())
+            _native, _handle = module, lib
+    return _handle
+
+
+def _import_native():
+    name = f"{__package__}._native"
+    importlib.invalidate_caches()  # (the file may be younger than the folder's cached listing)
+    try:
+        return importlib.import_module(name)
+    except ModuleNotFoundError as error:  # (any other failure to import it is not a missing build, and says what it is)
+        if error.name != name:
+            raise
+        raise RuntimeError("sage_b200/_native.so is missing: build it with `python -m sage_b200.build`") from None
+
+
+def _bind_library() -> ctypes.CDLL:
+    """The shared library with its functions' types."""
     lib = ctypes.CDLL(str(LIBRARY))
     vp, ci, sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
     lib.sageb200_version.restype = ci
@@ -381,46 +406,71 @@ def load() -> ctypes.CDLL:
     lib.sageb200_peer_all_reduce.argtypes = [ctypes.POINTER(vp), ci, ci, ll, vp, ll, vp]
     if "SAGEB200_PDL" in os.environ:  # debug switch: which kernel families launch dependently
         lib.sageb200_set_pdl(int(os.environ["SAGEB200_PDL"]))
-    native_module().bind({name: ctypes.cast(getattr(lib, name), vp).value for name in NATIVE_SYMBOLS})
-    _handle = lib
     return lib
 
 
 def register_operator(name: str, schema: str, fake):
     """Define `wvq::<name>` (or `sage_b200::<name>` when the reference package already owns the former in
     this process) with its fake kernel; the CUDA and autograd kernels are the C++ side's."""
-    tags = (torch.Tag.pt2_compliant_tag, torch.Tag.needs_fixed_stride_order)
     for namespace in ("wvq", "sage_b200"):
         try:
-            library = torch.library.Library(namespace, "FRAGMENT")
-            library.define(name + schema, tags=tags)
+            library = _define(namespace, name, schema)
             break
         except RuntimeError:
             if namespace == "sage_b200":
                 raise
-    torch.library.register_fake(f"{namespace}::{name}", fake, lib=library)
-    _libraries.append(library)
-    if native is not None:
-        native.register_kernels(name, namespace)
-    else:
-        library.impl(name, lambda *args: native_module(), "CUDA")
-    return getattr(getattr(torch.ops, namespace), name).default
+    return _set_kernels(library, namespace, name, fake, derivative=True)
 
 
 def register_typed_operator():
     """`sage_b200::linear`: a packed linear of FP16 or BF16 rows with its bias, the module's whole arithmetic in one
     operator (internal: the modules call it where no derivative is asked for)."""
-    library = torch.library.Library("sage_b200", "FRAGMENT")
-    library.define("linear(Tensor x, Tensor packed_codes, Tensor radius_codes, Tensor radius_grid, Tensor codebook, "
-                   "Tensor permutation, SymInt out_features, Tensor? bias) -> Tensor",
-                   tags=(torch.Tag.pt2_compliant_tag, torch.Tag.needs_fixed_stride_order))
-    torch.library.register_fake("sage_b200::linear", lambda x, codes, radii, grid, book, perm, n, bias:
-                                x.new_empty((*x.shape[:-1], n)), lib=library)
+    library = _define("sage_b200", "linear",
+                      "(Tensor x, Tensor packed_codes, Tensor radius_codes, Tensor radius_grid, Tensor codebook, "
+                      "Tensor permutation, SymInt out_features, Tensor? bias) -> Tensor")
+    _set_kernels(library, "sage_b200", "linear", lambda x, codes, radii, grid, book, perm, n, bias:
+                 x.new_empty((*x.shape[:-1], n)), derivative=False)
+
+
+def _define(namespace: str, name: str, schema: str) -> torch.library.Library:
+    library = torch.library.Library(namespace, "FRAGMENT")
+    library.define(name + schema, tags=(torch.Tag.pt2_compliant_tag, torch.Tag.needs_fixed_stride_order))
+    return library
+
+
+def _set_kernels(library: torch.library.Library, namespace: str, name: str, fake, *, derivative: bool):
+    torch.library.register_fake(f"{namespace}::{name}", fake, lib=library)
+    op = getattr(getattr(torch.ops, namespace), name).default
+
+    # The C++ kernels take the CUDA key, and AutogradCUDA where `derivative`, once `load` has registered them.  Until
+    # then a call lands on one of these two, which load them and dispatch again; afterwards only what has no kernel
+    # still does (theirs are the general keys, which a key's own kernel goes before).
+    def autograd(*args):
+        if _native is None and LIBRARY.exists():
+            load()
+            return op(*args)
+        with torch._C._AutoDispatchBelowAutograd():
+            return op(*args)
+
+    def backend(*args):
+        if _native is None:
+            load()
+            return op(*args)
+        raise NotImplementedError(f"Could not run '{namespace}::{name}' on {args[0].device}: it has a CUDA kernel only")
+
+    if derivative:
+        library.impl(name, autograd, "Autograd")
+    library.impl(name, backend, "CompositeExplicitAutograd")
     _libraries.append(library)
-    if native is not None:
-        native.register_kernels("linear", "sage_b200")
+    with _load_lock:
+        if _native is None:
+            _unregistered.append((name, namespace))
+        else:
+            _native.register_kernels(name, namespace)
+    return op
 
 
+_unregistered: list = []  # operators whose C++ kernels `load` has still to register
 _libraries: list = []  # the registrations live as long as the process
 
 

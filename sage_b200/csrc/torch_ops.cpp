@@ -570,10 +570,10 @@ PyObject *py_register_kernels(PyObject *, PyObject *const *a, Py_ssize_t count) 
   op_namespace[sage ? 0 : 1] = space;
   if (sage) {
     library(c10::DispatchKey::CUDA).impl("sage", &sage_cuda);
-    library(c10::DispatchKey::Autograd).impl("sage", &sage_autograd);
+    library(c10::DispatchKey::AutogradCUDA).impl("sage", &sage_autograd);
   } else {
     library(c10::DispatchKey::CUDA).impl("sphquant", &sph_run);
-    library(c10::DispatchKey::Autograd).impl("sphquant", &sph_autograd);
+    library(c10::DispatchKey::AutogradCUDA).impl("sphquant", &sph_autograd);
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS

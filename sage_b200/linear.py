@@ -16,7 +16,12 @@ from torch import nn
 from . import _lib
 from .ops import sage, sage_dequantize
 
-_sage_module = getattr(_lib.native, "sage_module", lambda *args: _lib.native_module())
+
+def _sage_module(*args):
+    """The native call; the first one puts it in this name's place (a look-up per call is host time of a small call)."""
+    global _sage_module
+    _sage_module = _lib.native_module().sage_module
+    return _sage_module(*args)
 
 
 class SAGELinear(nn.Module):

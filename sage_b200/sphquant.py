@@ -41,7 +41,13 @@ sphquant = _lib.register_operator(
     "-> Tensor",
     _fake,
 )
-_sph_module = getattr(_lib.native, "sph_module", lambda *args: _lib.native_module())
+
+
+def _sph_module(*args):
+    """The native call; the first one puts it in this name's place (a look-up per call is host time of a small call)."""
+    global _sph_module
+    _sph_module = _lib.native_module().sph_module
+    return _sph_module(*args)
 
 
 def sph_dequantize(packed_codes, radius_extra, radius_scales, radius_mins, codebook) -> torch.Tensor:
