@@ -241,11 +241,15 @@ def _import_native():
     name = f"{__package__}._native"
     importlib.invalidate_caches()  # (the file may be younger than the folder's cached listing)
     try:
-        return importlib.import_module(name)
+        module = importlib.import_module(name)
     except ModuleNotFoundError as error:  # (any other failure to import it is not a missing build, and says what it is)
         if error.name != name:
             raise
         raise RuntimeError("sage_b200/_native.so is missing: build it with `python -m sage_b200.build`") from None
+    if module.torch_version != str(torch.__version__):
+        raise RuntimeError(f"sage_b200/_native.so was built for torch {module.torch_version} and this is torch "
+                           f"{torch.__version__}: build it again with `python -m sage_b200.build`")
+    return module
 
 
 def _bind_library() -> ctypes.CDLL:

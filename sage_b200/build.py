@@ -64,9 +64,21 @@ def _older(target: pathlib.Path, inputs: list[pathlib.Path]) -> bool:
     return any(path.stat().st_mtime > built for path in inputs)
 
 
+def _library_stale() -> bool:
+    return _older(LIBRARY, [*sources(), *_inputs()])
+
+
+def _native_stale() -> bool:
+    """Older than its sources, or not to be had by a fresh interpreter: torch's C++ interface has no stable ABI, so a
+    module that another torch version was built against may miss symbols, or worse, find them."""
+    if _older(NATIVE, [CSRC / "torch_ops.cpp", *_inputs()]):
+        return True
+    check = f"from {PACKAGE.name} import _lib; _lib._import_native()"
+    return subprocess.run([sys.executable, "-c", check], cwd=PACKAGE.parent, capture_output=True).returncode != 0
+
+
 def is_stale() -> bool:
-    native = CSRC / "torch_ops.cpp"
-    return _older(LIBRARY, [*sources(), *_inputs()]) or _older(NATIVE, [native, *_inputs()])
+    return _library_stale() or _native_stale()
 
 
 def _run(command: list[str], what: str, verbose: bool) -> str:
@@ -87,7 +99,8 @@ def _build_native(verbose: bool) -> None:
     includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include",
                 pathlib.Path(_nvcc()).resolve().parent.parent / "include", sysconfig.get_paths()["include"]]
     command = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
-               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f'-DSAGEB200_TORCH_VERSION="{torch.__version__}"']
     for path in includes:
         command += ["-isystem", str(path)]
     command += [str(CSRC / "torch_ops.cpp"), "-o", str(NATIVE), f"-L{root / 'lib'}",
@@ -99,7 +112,8 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> pa
     """Compile every .cu under csrc/ into one shared library; returns its path.  `trace` adds
     -DSAGEB200_TRACE: the decode kernel's phase clocks (sageb200_debug_trace) and the
     SAGEB200_PATHS switch, both compiled out of the default build."""
-    if not force and not trace and not is_stale():
+    native_stale = not trace and (force or _native_stale())
+    if not force and not trace and not native_stale and not _library_stale():
         return LIBRARY
     flags = NVCC_FLAGS + (["-DSAGEB200_TRACE"] if trace else [])
     # the profiling build goes beside the product library (select it with SAGEB200_LIBRARY)
@@ -115,9 +129,7 @@ def build(force: bool = False, verbose: bool = False, trace: bool = False) -> pa
         return out, log.read_text()
 
     with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
-        native = None
-        if not trace and (force or _older(NATIVE, [CSRC / "torch_ops.cpp", *_inputs()])):
-            native = pool.submit(_build_native, verbose)
+        native = pool.submit(_build_native, verbose) if native_stale else None
         done = list(pool.map(compile_one, sources()))
         if native is not None:
             native.result()

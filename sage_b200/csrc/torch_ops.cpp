@@ -599,4 +599,9 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__native() {
+  PyObject *module = PyModule_Create(&module_def);
+  // (torch's C++ interface has no stable ABI: the loader compares this with the torch it runs under)
+  if (module && PyModule_AddStringConstant(module, "torch_version", SAGEB200_TORCH_VERSION) < 0) Py_CLEAR(module);
+  return module;
+}

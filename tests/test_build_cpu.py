@@ -89,3 +89,48 @@ assert torch._C._dispatch_has_kernel_for_dispatch_key(sage_b200.sphquant.name(),
     maps = "print(sum('sage_b200' in line and '.so' in line for line in open('/proc/self/maps')))"
     assert run(f"import sage_b200\n{maps}", unbuilt).strip() == "0"
     assert int(run(f"from sage_b200 import _lib\n_lib.load()\n{maps}", unbuilt)) > 0
+
+
+@pytest.fixture
+def built(tmp_path):
+    """The package with its built files, newer than every source."""
+    from sage_b200 import build
+
+    build.build()
+    shutil.copytree(ROOT / "sage_b200", tmp_path / "sage_b200", ignore=shutil.ignore_patterns("_obj", "__pycache__"))
+    shutil.copytree(ROOT / "include", tmp_path / "include")
+    for name in ("libsage_b200.so", "_native.so"):
+        (tmp_path / "sage_b200" / name).touch()
+    return tmp_path
+
+
+STALE = "from sage_b200 import build; print(build._native_stale())"
+
+
+def test_a_module_that_does_not_import_says_why_and_is_built_again(built):
+    assert run(STALE, built).strip() == "False"
+    (built / "sage_b200" / "_native.so").write_bytes(b"not a shared object")
+    run("""
+from sage_b200 import _lib
+try:
+    _lib.load()
+except ImportError as error:  # the loader's own words, not "missing"
+    assert "missing" not in str(error) and "_native.so" in str(error), error
+else:
+    raise AssertionError("loaded")
+""", built)
+    assert run(STALE, built).strip() == "True"
+
+
+def test_a_module_of_another_torch_version_is_refused(built):
+    run("""
+import torch
+torch.__version__ = "0.0"  # as if torch had been exchanged after the build
+from sage_b200 import _lib
+try:
+    _lib._import_native()  # (what the build's check of an existing module calls as well)
+except RuntimeError as error:
+    assert "torch 0.0" in str(error) and "python -m sage_b200.build" in str(error), error
+else:
+    raise AssertionError("loaded")
+""", built)
