@@ -19,6 +19,7 @@
 #include "sage_common.cuh"
 #include "sage_kernels.h"
 #include "sage_rows.cuh"
+#include "shared_opt_in.h"
 
 namespace {
 
@@ -2109,13 +2110,9 @@ int sageb200_glue_add_rmsnorm_permuted(void *residual, const void *delta, const 
       (reinterpret_cast<uintptr_t>(delta) & 15) == 0) {
     const int blocks = (rows + sageb200::kRowsAtOnce - 1) / sageb200::kRowsAtOnce;
     const size_t bytes = static_cast<size_t>((hidden + 127) / 128 * 128) * sizeof(uint2);
-    static bool four_configured = false;
-    if (!four_configured) {
-      if (cudaFuncSetAttribute(add_rmsnorm_permuted_four_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               12800 * sizeof(uint2)) != cudaSuccess)
-        return -5;
-      four_configured = true;
-    }
+    static sageb200::SharedOptIn opt_in;
+    if (opt_in(reinterpret_cast<const void *>(add_rmsnorm_permuted_four_kernel), 12800 * sizeof(uint2)) != cudaSuccess)
+      return -5;
     sageb200::launch_dependent<2>(add_rmsnorm_permuted_four_kernel, blocks, kNormThreads, bytes,
                                   static_cast<cudaStream_t>(stream), static_cast<__half *>(residual),
                                   static_cast<const __half *>(delta), static_cast<const __half *>(weight),
@@ -2123,13 +2120,9 @@ int sageb200_glue_add_rmsnorm_permuted(void *residual, const void *delta, const 
     return launch_status();
   }
   const size_t shared = hidden * sizeof(__half);
-  static bool configured = false;
-  if (shared > 40 * 1024 && !configured) {
-    if (cudaFuncSetAttribute(add_rmsnorm_permuted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) !=
-        cudaSuccess)
-      return -5;
-    configured = true;
-  }
+  static sageb200::SharedOptIn opt_in;
+  if (shared > 40 * 1024 && opt_in(reinterpret_cast<const void *>(add_rmsnorm_permuted_kernel), 64 * 1024) != cudaSuccess)
+    return -5;
   sageb200::launch_dependent<1, true>(add_rmsnorm_permuted_kernel, rows, kNormThreads, shared,
                                 static_cast<cudaStream_t>(stream), static_cast<__half *>(residual),
                                 static_cast<const __half *>(delta), static_cast<const __half *>(weight),
@@ -2146,13 +2139,8 @@ int sageb200_glue_swiglu_permuted(const void *gate, const void *up, const void *
   if (rows >= kManyRows && k <= 25600) {
     const int blocks = (rows + sageb200::kRowsAtOnce - 1) / sageb200::kRowsAtOnce;
     const size_t bytes = static_cast<size_t>((k + 127) / 128 * 128) * sizeof(uint2);
-    static bool four_configured = false;
-    if (!four_configured) {
-      if (cudaFuncSetAttribute(swiglu_permuted_four_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               25600 * sizeof(uint2)) != cudaSuccess)
-        return -5;
-      four_configured = true;
-    }
+    static sageb200::SharedOptIn opt_in;
+    if (opt_in(reinterpret_cast<const void *>(swiglu_permuted_four_kernel), 25600 * sizeof(uint2)) != cudaSuccess) return -5;
     sageb200::launch_dependent<2>(swiglu_permuted_four_kernel, blocks, kSwigluFourThreads, bytes,
                                   static_cast<cudaStream_t>(stream), static_cast<const __half *>(gate),
                                   static_cast<const __half *>(up), static_cast<const int *>(perm),
@@ -2160,13 +2148,9 @@ int sageb200_glue_swiglu_permuted(const void *gate, const void *up, const void *
     return launch_status();
   }
   const size_t shared = static_cast<size_t>(k) * sizeof(__half);
-  static bool configured = false;
-  if (shared > 40 * 1024 && !configured) {
-    if (cudaFuncSetAttribute(swiglu_permuted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
-        cudaSuccess)
-      return -5;
-    configured = true;
-  }
+  static sageb200::SharedOptIn opt_in;
+  if (shared > 40 * 1024 && opt_in(reinterpret_cast<const void *>(swiglu_permuted_kernel), 200 * 1024) != cudaSuccess)
+    return -5;
   int blocks = rows;
   const int cap = (sm_count > 0 ? sm_count : 148) * 4;
   if (blocks > cap) blocks = cap;
@@ -2189,13 +2173,8 @@ int sageb200_glue_lm_head(const void *head, const void *x, void *logits, int row
   if (rows > 16 || hidden % 8) return -1;
   const int staged_rows = rows > 1 && hidden % 32 == 0 ? (rows > 8 ? 16 : 8) : rows;  // (blocked copy: whole column blocks)
   const size_t shared = static_cast<size_t>(staged_rows) * hidden * sizeof(__half);
-  static bool configured = false;
-  if (shared > 48 * 1024 && !configured) {
-    if (cudaFuncSetAttribute(lm_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
-        cudaSuccess)
-      return -5;
-    configured = true;
-  }
+  static sageb200::SharedOptIn opt_in;
+  if (shared > 48 * 1024 && opt_in(reinterpret_cast<const void *>(lm_head_kernel), 200 * 1024) != cudaSuccess) return -5;
   const int blocks = (sm_count > 0 ? sm_count : 148) * 4;
   sageb200::launch_dependent<2>(lm_head_kernel, blocks, kHeadWarps * 32, shared, static_cast<cudaStream_t>(stream),
       static_cast<const __half *>(head), static_cast<const __half *>(x), static_cast<__half *>(logits),
