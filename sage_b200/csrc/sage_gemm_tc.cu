@@ -730,17 +730,28 @@ __global__ void __launch_bounds__(kGatherFourThreads) sage_gather_four_kernel(co
 
 }  // namespace
 
+namespace {
+template <typename Function>
+Function driver_function(const char *name) {
+  void *symbol = nullptr;
+  cudaDriverEntryPointQueryResult query;
+  if (cudaGetDriverEntryPoint(name, &symbol, cudaEnableDefault, &query) != cudaSuccess || query != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return reinterpret_cast<Function>(symbol);
+}
+}  // namespace
+
+// The driver's call crashes on a thread without a current context.  The runtime binds one at a thread's first launch,
+// but the maps are made before the launch, so a thread whose first GPU work this is has none yet: bind it here.
 EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void *symbol = nullptr;
-    cudaDriverEntryPointQueryResult query;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &symbol, cudaEnableDefault, &query) ==
-            cudaSuccess &&
-        query == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(symbol);
-  }
-  return fn;
+  static const auto encode = driver_function<EncodeTiledFn>("cuTensorMapEncodeTiled");
+  static const auto current = driver_function<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
+  if (!encode || !current) return nullptr;
+  CUcontext context = nullptr;
+  if (current(&context) == CUDA_SUCCESS && context) return encode;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return nullptr;
+  return current(&context) == CUDA_SUCCESS && context ? encode : nullptr;
 }
 
 namespace {
