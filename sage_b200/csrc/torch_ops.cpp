@@ -72,33 +72,46 @@ void check_bound() {
 constexpr int64_t kCounterRegion = 64 * 1024;  // the front of the scratch that has to be zero
 constexpr int kMaxDevices = 64;
 
-// The default stream's scratch, one zero-filled buffer per device, grown on demand (the kernels
-// leave its counters zero).  Calls on that stream run in order, so all threads share it; a buffer
-// that was outgrown goes back to the caching allocator, which reuses it in stream order, and no
-// captured graph can hold it because the default stream cannot be captured.
-std::mutex scratch_mutex;
-Tensor *scratch_of_device() {
-  static auto *buffers = new Tensor[kMaxDevices];  // never destroyed: the allocator may be gone by then
-  return buffers;
+// The default stream's scratch: one zero-filled buffer per device for all threads, grown on demand (the kernels leave
+// its counters zero).  A call is several launches that hand data to one another through the buffer (gather or staging,
+// then the matmul), so it keeps the device's lock until all of them are enqueued: another thread's call then comes
+// behind it on the stream and finds the buffer free.  A buffer that was outgrown goes back to the caching allocator,
+// which reuses it in stream order, and no captured graph can hold it because the default stream cannot be captured.
+struct SharedScratch {
+  std::mutex mutex;
+  Tensor buffer;
+};
+SharedScratch &shared_scratch(int device) {
+  static auto *all = new SharedScratch[kMaxDevices];  // never destroyed: the allocator may be gone by then
+  return all[device];
 }
 
-Tensor default_scratch(const Tensor &x, int64_t bytes) {
-  std::lock_guard<std::mutex> lock(scratch_mutex);
-  Tensor &buffer = scratch_of_device()[x.get_device()];
-  if (!buffer.defined() || buffer.numel() < bytes)
-    buffer = at::zeros({std::max<int64_t>(bytes, kCounterRegion)}, x.options().dtype(at::kByte));
-  return buffer;
-}
+// Scratch of one call; lives until the call's launches are enqueued.
+struct Scratch {
+  Tensor buffer;                     // undefined for a call that needs none
+  std::unique_lock<std::mutex> use;  // held where the buffer is a shared one
+  void *data() const { return buffer.defined() ? buffer.data_ptr() : nullptr; }
+  size_t bytes() const { return buffer.defined() ? static_cast<size_t>(buffer.numel()) : 0; }
+};
 
-// Scratch of a call that brings none; undefined for 0 bytes.
-Tensor scratch_for(const Tensor &x, int64_t bytes, cudaStream_t stream) {
-  if (bytes == 0) return Tensor();
-  if (stream == nullptr) return default_scratch(x, bytes);
+// Scratch of a call that brings none.
+Scratch scratch_for(const Tensor &x, int64_t bytes, cudaStream_t stream) {
+  Scratch scratch;
+  if (bytes == 0) return scratch;
+  const auto options = x.options().dtype(at::kByte);
+  if (stream == nullptr) {
+    SharedScratch &shared = shared_scratch(x.get_device());
+    scratch.use = std::unique_lock<std::mutex>(shared.mutex);
+    if (!shared.buffer.defined() || shared.buffer.numel() < bytes)
+      shared.buffer = at::zeros({std::max<int64_t>(bytes, kCounterRegion)}, options);
+    scratch.buffer = shared.buffer;
+    return scratch;
+  }
   // Any other stream may be under capture, or belong to a compiled graph whose memory pool accepts
   // no allocation that outlives the call: a temporary of this call, its counters zeroed.
-  Tensor workspace = at::empty({bytes}, x.options().dtype(at::kByte));
-  C10_CUDA_CHECK(cudaMemsetAsync(workspace.data_ptr(), 0, std::min(bytes, kCounterRegion), stream));
-  return workspace;
+  scratch.buffer = at::empty({bytes}, options);
+  C10_CUDA_CHECK(cudaMemsetAsync(scratch.buffer.data_ptr(), 0, std::min(bytes, kCounterRegion), stream));
+  return scratch;
 }
 
 bool shape_is(const Tensor &t, std::initializer_list<int64_t> want) {
@@ -152,19 +165,18 @@ Tensor sage_run(const Tensor &x, const Tensor &codes, const Tensor &radii, const
   TORCH_CHECK(rows <= 65535, "SAGE launch dimensions exceed supported range");
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
   const int64_t bytes = static_cast<int64_t>(abi.workspace_bytes(static_cast<int>(rows), static_cast<int>(n), static_cast<int>(k)));
-  Tensor workspace;
+  Scratch workspace;
   if (bytes && scratch) {
     TORCH_CHECK(scratch->device() == x.device() && scratch->scalar_type() == at::kByte && scratch->numel() >= bytes,
                 "SAGE scratch must be a uint8 tensor of at least ", bytes, " bytes on the input device");
-    workspace = *scratch;
+    workspace.buffer = *scratch;
   } else {
     workspace = scratch_for(x, bytes, stream);
   }
   check_status(abi.linear(x.data_ptr(), codes.data_ptr(), radii.data_ptr(), grid.data_ptr(), book.data_ptr(),
                           perm.numel() ? perm.data_ptr<int32_t>() : nullptr, y.data_ptr(),
-                          workspace.defined() ? workspace.data_ptr() : nullptr,
-                          workspace.defined() ? static_cast<size_t>(workspace.numel()) : 0, static_cast<int>(rows),
-                          static_cast<int>(n), static_cast<int>(k), static_cast<int>(book.size(1)), stream));
+                          workspace.data(), workspace.bytes(), static_cast<int>(rows), static_cast<int>(n),
+                          static_cast<int>(k), static_cast<int>(book.size(1)), stream));
   return y;
 }
 
@@ -189,12 +201,11 @@ Tensor sph_run(const Tensor &x, const Tensor &codes, const Tensor &extra, const 
   const int64_t rows = x.numel() / k;
   if (rows == 0 || n == 0) return y;
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
-  const Tensor workspace =
+  const Scratch workspace =
       scratch_for(x, static_cast<int64_t>(abi.sph_workspace_bytes(static_cast<int>(rows), static_cast<int>(n), static_cast<int>(k))), stream);
   check_status(abi.sph_linear_scratch(x.data_ptr(), codes.data_ptr(), extra.data_ptr(), scales.data_ptr(), mins.data_ptr(),
-                                      book.data_ptr(), y.data_ptr(), workspace.defined() ? workspace.data_ptr() : nullptr,
-                                      workspace.defined() ? static_cast<size_t>(workspace.numel()) : 0,
-                                      static_cast<int>(rows), static_cast<int>(n), static_cast<int>(k), stream));
+                                      book.data_ptr(), y.data_ptr(), workspace.data(), workspace.bytes(), static_cast<int>(rows),
+                                      static_cast<int>(n), static_cast<int>(k), stream));
   return y;
 }
 
@@ -313,14 +324,13 @@ Tensor linear_run(const Tensor &x, const Tensor &codes, const Tensor &radii, con
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor y = empty_output(x, n);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
-    const Tensor workspace = scratch_for(
+    const Scratch workspace = scratch_for(
         x, static_cast<int64_t>(abi.workspace_bytes(static_cast<int>(rows), static_cast<int>(n), static_cast<int>(k))), stream);
     check_status(abi.linear_typed(x.data_ptr(), type == at::kBFloat16, codes.data_ptr(), radii.data_ptr(), grid.data_ptr(),
                                   book.data_ptr(), perm.numel() ? perm.data_ptr<int32_t>() : nullptr,
                                   bias.defined() ? bias.data_ptr() : nullptr, y.data_ptr(),
-                                  workspace.defined() ? workspace.data_ptr() : nullptr,
-                                  workspace.defined() ? static_cast<size_t>(workspace.numel()) : 0, static_cast<int>(rows),
-                                  static_cast<int>(n), static_cast<int>(k), static_cast<int>(book.size(1)), stream));
+                                  workspace.data(), workspace.bytes(), static_cast<int>(rows), static_cast<int>(n),
+                                  static_cast<int>(k), static_cast<int>(book.size(1)), stream));
     return y;
   }
   return finish(sage_run(to_half(x), codes, radii, grid, book, perm, n, nullptr), type, bias);

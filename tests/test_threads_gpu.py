@@ -35,3 +35,42 @@ def test_first_gpu_work_of_a_thread_is_a_tensor_map(make):
     thread.join()
     torch.cuda.synchronize()
     assert len(got) == 1 and torch.equal(want, got[0])
+
+
+# calls of several launches through the scratch: gather and GEMM with and without K splits, staging and decode kernel
+# with K slices, the second format's splits
+CASES = {
+    "gather_gemm": (sage, 2560, 1024, (33, 300, 64, 513)),
+    "gather_split_gemm": (sage, 4096, 256, (48, 40, 130, 65)),
+    "staging_sliced_decode": (sage, 9728, 512, (16, 9, 12, 8)),
+    "sph_split_gemm": (sph, 4096, 256, (40, 64, 100, 33)),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_threads_on_the_default_stream_do_not_share_scratch(name):
+    make, k, n, rows = CASES[name]
+    layers = [make(k, n, seed) for seed in range(len(rows))]
+    inputs = [rows_of(m, k) for m in rows]
+    alone = [layer(x) for layer, x in zip(layers, inputs)]
+    torch.cuda.synchronize()
+    outputs, errors = [[] for _ in rows], []
+    start = threading.Barrier(len(rows))
+
+    def work(i):
+        try:
+            start.wait()
+            for _ in range(200):
+                outputs[i].append(layers[i](inputs[i]))
+        except Exception as error:  # noqa: BLE001 - reported by the test's own thread
+            errors.append(error)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(rows))]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    for want, got in zip(alone, outputs):  # (partial sums are added in a fixed order: the same bits)
+        assert all(torch.equal(want, y) for y in got)
