@@ -30,7 +30,7 @@ import torch
 from torch import nn
 
 from . import _lib
-from .ops import _workspace
+from .ops import _WORKSPACE_LOCK, _workspace
 from .synthetic import synthetic_sage_device
 
 STACK_KEYS = ("packed_codes", "radius_codes", "radius_grid", "codebook", "permutation")
@@ -254,11 +254,12 @@ class SAGEExperts(nn.Module):
 
     def _run(self, lib, x: int, stride: int, stacks, ys, ids: torch.Tensor, slots: int, stream: int):
         need = lib.sageb200_experts_workspace_bytes(stacks, len(stacks), slots)
-        workspace = _workspace(ids.device, stream, need) if need else None
-        _lib.check(lib.sageb200_experts(
-            x, stride, stacks, ys, len(stacks), ids.data_ptr(), slots,
-            workspace.data_ptr() if workspace is not None else None,
-            workspace.numel() if workspace is not None else 0, stream))
+        with _WORKSPACE_LOCK:
+            workspace = _workspace(ids.device, stream, need) if need else None
+            _lib.check(lib.sageb200_experts(
+                x, stride, stacks, ys, len(stacks), ids.data_ptr(), slots,
+                workspace.data_ptr() if workspace is not None else None,
+                workspace.numel() if workspace is not None else 0, stream))
 
     def forward_blocks(self, rows: torch.Tensor, block_experts: torch.Tensor) -> torch.Tensor:
         """rows FP16 [blocks, r <= 16, hidden], block_experts int32 [blocks] (global expert ids on the
@@ -292,11 +293,12 @@ class SAGEExperts(nn.Module):
             ys = (ctypes.c_void_p * len(outputs))(*[out.data_ptr() for out in outputs])
             stream = torch.cuda.current_stream(x.device).cuda_stream
             need = lib.sageb200_expert_blocks_workspace_bytes(array, len(stacks), count)
-            workspace = _workspace(x.device, stream, need) if need else None
-            _lib.check(lib.sageb200_expert_blocks(
-                x.data_ptr(), array, ys, len(stacks), ids.data_ptr(), blocks, count,
-                workspace.data_ptr() if workspace is not None else None,
-                workspace.numel() if workspace is not None else 0, stream))
+            with _WORKSPACE_LOCK:
+                workspace = _workspace(x.device, stream, need) if need else None
+                _lib.check(lib.sageb200_expert_blocks(
+                    x.data_ptr(), array, ys, len(stacks), ids.data_ptr(), blocks, count,
+                    workspace.data_ptr() if workspace is not None else None,
+                    workspace.numel() if workspace is not None else 0, stream))
 
         with torch.cuda.device(rows.device):
             stream = torch.cuda.current_stream(rows.device).cuda_stream

@@ -14,6 +14,7 @@ Argument checks and their messages follow the reference's native entry point
 from __future__ import annotations
 
 import ctypes
+import threading
 
 import torch
 
@@ -21,6 +22,9 @@ from . import _lib
 
 _WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
 _RETIRED: list[torch.Tensor] = []  # outgrown buffers a captured graph may still point at
+# Held from fetching a buffer until the call's launches are enqueued: threads on one stream share its buffer, a call is
+# several launches that hand data to one another through it, and ctypes runs it without the interpreter's lock.
+_WORKSPACE_LOCK = threading.Lock()
 
 
 def _workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
@@ -161,7 +165,7 @@ def sage_grouped(problems: list[tuple], out_features: list[int], activation: tup
             x.data_ptr(), codes.data_ptr(), radii.data_ptr(), grid.data_ptr(), book.data_ptr(),
             perm.data_ptr() if perm.numel() else None, y.data_ptr(), rows, n, k, book.shape[1],
         )
-    with torch.cuda.device(device):
+    with torch.cuda.device(device), _WORKSPACE_LOCK:
         stream = torch.cuda.current_stream(device).cuda_stream
         if activation is None:
             total = lib.sageb200_grouped_workspace_bytes(array, len(problems))

@@ -5,7 +5,7 @@ import threading
 import pytest
 import torch
 
-from sage_b200 import SAGELinear, SPHQuantLinear, synthetic_sage, synthetic_sphquant
+from sage_b200 import SAGELinear, SPHQuantLinear, sage_grouped, synthetic_sage, synthetic_sphquant
 
 pytestmark = pytest.mark.gpu
 
@@ -37,13 +37,25 @@ def test_first_gpu_work_of_a_thread_is_a_tensor_map(make):
     assert len(got) == 1 and torch.equal(want, got[0])
 
 
+class Grouped:
+    """Two linears of one input in a grouped call, a staging and a decode launch."""
+
+    def __init__(self, k, n, seed):
+        self.packed, self.n = [list(synthetic_sage(k, n, seed=seed + i).values()) for i in range(2)], n
+        self.packed = [[value.cuda() for value in values] for values in self.packed]
+
+    def __call__(self, x):
+        return torch.stack(sage_grouped([(x, *values) for values in self.packed], [self.n] * 2))
+
+
 # calls of several launches through the scratch: gather and GEMM with and without K splits, staging and decode kernel
-# with K slices, the second format's splits
+# with K slices, the second format's splits, grouped problems
 CASES = {
     "gather_gemm": (sage, 2560, 1024, (33, 300, 64, 513)),
     "gather_split_gemm": (sage, 4096, 256, (48, 40, 130, 65)),
     "staging_sliced_decode": (sage, 9728, 512, (16, 9, 12, 8)),
     "sph_split_gemm": (sph, 4096, 256, (40, 64, 100, 33)),
+    "grouped": (Grouped, 2560, 512, (16, 9, 12, 3)),
 }
 
 
