@@ -276,11 +276,12 @@ int sageb200_pack_logits(const void *signs, const void *indices, int index_bytes
 /*
  * The small tensors beside it.  Codebook: FP32 logits [entries][7] -> unit directions, FP16, theta = offset +
  * scale * sigmoid(logit); planar != 0: [4][entries][2], else [entries][8].  Permutation: int64 order [k] ->
- * int32 inverse [k]; *moved (int32, zeroed by the caller) becomes 1 where order is not the identity.
+ * int32 inverse [k], every entry of it a channel whatever the order holds; *verdict (int32): bit 0 where order is not
+ * the identity, bit 1 where it is no permutation (an entry out of range or twice) and the inverse is of no use.
  */
 int sageb200_codebook_logits(const void *angle_logits, void *book, int entries, float scale, float offset, int planar,
                              void *stream);
-int sageb200_invert_permutation(const void *order, void *inverse, void *moved, int k, void *stream);
+int sageb200_invert_permutation(const void *order, void *inverse, void *verdict, int k, void *stream);
 
 /*
  * Host-buffer form of sageb200_linear for callers whose activations live in host

@@ -1012,10 +1012,10 @@ int sageb200_codebook_logits(const void *angle_logits, void *book, int entries, 
   return SAGEB200_OK;
 }
 
-int sageb200_invert_permutation(const void *order, void *inverse, void *moved, int k, void *stream) {
-  if (k <= 0 || !order || !inverse || !moved) return SAGEB200_ERR_INVALID_ARGUMENT;
+int sageb200_invert_permutation(const void *order, void *inverse, void *verdict, int k, void *stream) {
+  if (k <= 0 || !order || !inverse || !verdict) return SAGEB200_ERR_INVALID_ARGUMENT;
   if (launch_invert_permutation(static_cast<const long long *>(order), static_cast<int *>(inverse),
-                                static_cast<int *>(moved), k, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
+                                static_cast<int *>(verdict), k, static_cast<cudaStream_t>(stream)) != cudaSuccess) {
     cudaGetLastError();
     return SAGEB200_ERR_CUDA;
   }

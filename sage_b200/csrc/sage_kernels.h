@@ -113,7 +113,7 @@ cudaError_t launch_pack(const int8_t *signs, const void *indices, int index_byte
 // Direction codebook of angular logits [entries][7]; inverse of a permutation (`moved`: zeroed by the caller).
 cudaError_t launch_codebook(const float *logits, __half *book, int entries, float scale, float offset, bool planar,
                             cudaStream_t stream);
-cudaError_t launch_invert_permutation(const long long *order, int *inverse, int *moved, int k, cudaStream_t stream);
+cudaError_t launch_invert_permutation(const long long *order, int *inverse, int *verdict, int k, cudaStream_t stream);
 
 // Per-device set-up of the library on the current device (idempotent): the device-visible
 // status word the kernels write on a timed-out wait, and the SM count.  Returns a

@@ -231,7 +231,8 @@ struct Packed {
 };
 
 // `order` (int64, optional): the checkpoint's inverse permutation.  Whether it is the identity decides what is
-// returned, so the host has to know it; it is inverted first and its answer read while the packing runs.
+// returned, and one that is no permutation is refused (the kernels index with its inverse unchecked), so the host has
+// to know; it is inverted first and the verdict read while the packing runs.
 Packed pack_state(const Tensor &signs, const Tensor &indices, const Tensor &radius_logits, const Tensor &angle_logits,
                   const Tensor &order, bool sage, double scale, double offset) {
   check_bound();
@@ -251,24 +252,23 @@ Packed pack_state(const Tensor &signs, const Tensor &indices, const Tensor &radi
   Packed out;
   // (one pinned word and event per thread and device, kept: an answer is read before the call returns)
   struct Answer {
-    int *moved = nullptr;
+    int *verdict = nullptr;
     cudaEvent_t event = nullptr;
   };
   static thread_local Answer answers[kMaxDevices];
   Answer &answer = answers[signs.get_device()];
-  Tensor moved;
+  Tensor verdict;
   if (order.defined()) {
     TORCH_CHECK(order.device() == signs.device() && order.scalar_type() == at::kLong && order.is_contiguous() && order.numel() == k,
                 "invalid channel permutation");
-    if (!answer.moved) {
-      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&answer.moved), sizeof(int), cudaHostAllocDefault));
+    if (!answer.verdict) {
+      C10_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void **>(&answer.verdict), sizeof(int), cudaHostAllocDefault));
       C10_CUDA_CHECK(cudaEventCreateWithFlags(&answer.event, cudaEventDisableTiming));
     }
     out.permutation = at::empty({k}, options.dtype(at::kInt));
-    moved = at::empty({1}, options.dtype(at::kInt));
-    C10_CUDA_CHECK(cudaMemsetAsync(moved.data_ptr(), 0, sizeof(int), stream));
-    check_status(abi.invert_permutation(order.data_ptr(), out.permutation.data_ptr(), moved.data_ptr(), static_cast<int>(k), stream));
-    C10_CUDA_CHECK(cudaMemcpyAsync(answer.moved, moved.data_ptr(), sizeof(int), cudaMemcpyDeviceToHost, stream));
+    verdict = at::empty({1}, options.dtype(at::kInt));
+    check_status(abi.invert_permutation(order.data_ptr(), out.permutation.data_ptr(), verdict.data_ptr(), static_cast<int>(k), stream));
+    C10_CUDA_CHECK(cudaMemcpyAsync(answer.verdict, verdict.data_ptr(), sizeof(int), cudaMemcpyDeviceToHost, stream));
     C10_CUDA_CHECK(cudaEventRecord(answer.event, stream));
   }
   if (sage) {
@@ -292,7 +292,8 @@ Packed pack_state(const Tensor &signs, const Tensor &indices, const Tensor &radi
                                static_cast<int>(k), static_cast<int>(entries), sage, stream));
   if (order.defined()) {
     C10_CUDA_CHECK(cudaEventSynchronize(answer.event));
-    if (*answer.moved == 0) out.permutation = Tensor();
+    TORCH_CHECK_VALUE((*answer.verdict & 2) == 0, "channel_unpermutation is not a permutation of the input channels");
+    if (*answer.verdict == 0) out.permutation = Tensor();
   }
   return out;
 }

@@ -8,6 +8,7 @@ import torch
 
 from oracle import pack_oracle
 from sage_b200 import sage_dequantize, sph_dequantize
+from sage_b200 import _lib
 from sage_b200.packing import direction_codebook_from_logits, pack_spherical, pack_spherical_radii
 from test_pack_oracle import CASES, packed_of
 
@@ -105,3 +106,45 @@ def test_pack_rejects_what_the_reference_rejects():
     state["radius_bits"] = torch.tensor(4)
     with pytest.raises(ValueError, match="bit split"):
         pack_spherical(state, sage=True)
+
+
+def spherical_state(n, k, order):
+    g = torch.Generator().manual_seed(k)
+    return {
+        "signs": (torch.randint(0, 2, (n, k), generator=g) * 2 - 1).to(torch.int8).cuda(),
+        "direction_indices": torch.randint(0, 64, (n, k // 8), generator=g).cuda(),
+        "radius_logits": torch.randn(n, k // 8, generator=g).cuda(),
+        "angle_logits": torch.randn(64, 7, generator=g).cuda(),
+        "radius_bits": torch.tensor(4), "group_size": torch.tensor(128), "sage_version": torch.tensor(1),
+        "channel_unpermutation": order.cuda(),
+    }
+
+
+@pytest.mark.parametrize("k", [128, 1024, 1152, 25600])
+def test_permutation_is_inverted(k):
+    order = torch.randperm(k, generator=torch.Generator().manual_seed(k))
+    packed = pack_spherical(spherical_state(16, k, order), sage=True)
+    assert torch.equal(packed["permutation"].cpu(), order.argsort().to(torch.int32))
+    swapped = torch.arange(k)
+    swapped[[0, k - 1]] = swapped[[k - 1, 0]]  # (two entries away from the identity)
+    assert torch.equal(pack_spherical(spherical_state(16, k, swapped), sage=True)["permutation"].cpu(), swapped.to(torch.int32))
+    assert pack_spherical(spherical_state(16, k, torch.arange(k)), sage=True)["permutation"].numel() == 0
+
+
+@pytest.mark.parametrize("k", [128, 2560])
+@pytest.mark.parametrize("at, value", [(0, 5), (127, 0), (3, -1), (3, 1 << 20), (3, 1 << 40)])
+def test_an_order_that_is_no_permutation_is_refused(k, at, value):
+    """An entry twice (and so another one never), or out of range: the kernels would index with whatever stands in
+    the inverse's gaps."""
+    for order in (torch.arange(k), torch.randperm(k, generator=torch.Generator().manual_seed(k))):
+        order[at] = value if value != order[at] else order[at + 1 if at + 1 < k else 0]
+        with pytest.raises(ValueError, match="not a permutation"):
+            pack_spherical(spherical_state(16, k, order), sage=True)
+    # the C entry by itself: every entry of the inverse is a channel
+    order = order.cuda()
+    inverse = torch.full((k,), -7, dtype=torch.int32, device="cuda")
+    verdict = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+    lib = _lib.load()
+    assert lib.sageb200_invert_permutation(order.data_ptr(), inverse.data_ptr(), verdict.data_ptr(), k,
+                                           torch.cuda.current_stream().cuda_stream) == 0
+    assert verdict.item() & 2 and 0 <= inverse.min().item() and inverse.max().item() < k
