@@ -154,12 +154,17 @@ __global__ void __launch_bounds__(kExpertThreads, 2) expert_mlp_kernel(const __g
         entry = make_uint4(__ldg(book + tid), __ldg(book + q.entries + tid), __ldg(book + 2 * q.entries + tid),
                            __ldg(book + 3 * q.entries + tid));
       const int32_t *perm = q.perm ? q.perm + static_cast<long long>(expert) * p.k : nullptr;
-      const int v0 = tid % vectors;
-      int4 lo = make_int4(v0 * 8, v0 * 8 + 1, v0 * 8 + 2, v0 * 8 + 3), hi = make_int4(v0 * 8 + 4, v0 * 8 + 5, v0 * 8 + 6, v0 * 8 + 7);
-      if (perm) {  // (whole int4s: K is a multiple of 128 and the stack is checked to be 16-byte aligned)
-        lo = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v0);
-        hi = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v0 + 1);
-      }
+      int held = tid % vectors;  // the vector whose source channels are in lo and hi
+      int4 lo, hi;
+      auto hold = [&](int v) {
+        held = v;
+        lo = make_int4(v * 8, v * 8 + 1, v * 8 + 2, v * 8 + 3), hi = make_int4(v * 8 + 4, v * 8 + 5, v * 8 + 6, v * 8 + 7);
+        if (perm) {  // (whole int4s: K is a multiple of 128 and the stack is checked to be 16-byte aligned)
+          lo = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v);
+          hi = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v + 1);
+        }
+      };
+      hold(held);
 
       __syncthreads();  // (everyone is done with the buffers of the matrix before)
       static_assert(kExpertThreads >= 256, "one codebook entry per thread");
@@ -188,13 +193,7 @@ __global__ void __launch_bounds__(kExpertThreads, 2) expert_mlp_kernel(const __g
       for (int i = tid; i < NB * vectors; i += kExpertThreads) {
         const int plane = NB == 1 ? 0 : i / vectors, v = i - plane * vectors;
         uint4 in[8], out[8];
-        if (v != v0) {
-          lo = make_int4(v * 8, v * 8 + 1, v * 8 + 2, v * 8 + 3), hi = make_int4(v * 8 + 4, v * 8 + 5, v * 8 + 6, v * 8 + 7);
-          if (perm) {
-            lo = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v);
-            hi = __ldg(reinterpret_cast<const int4 *>(perm) + 2 * v + 1);
-          }
-        }
+        if (v != held) hold(v);
         const int source[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
         for (int j = 0; j < 8; ++j)

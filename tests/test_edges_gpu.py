@@ -86,6 +86,30 @@ def test_expert_mlp_blocks(hidden, inter, experts, rows):
         assert ((got[b] - want).norm(dim=-1) / want.norm(dim=-1)).max() < 2e-3
 
 
+@pytest.mark.parametrize("hidden,inter", [(3328, 256), (256, 3328), (2176, 2048)])
+@pytest.mark.parametrize("rows", [8, 16])
+def test_expert_mlp_beyond_a_vector_per_thread(hidden, inter, rows):
+    """More than 2048 channels, up to the most that fit beside 64 entries with two operand blocks: threads come to
+    several vectors, and to another operand block's, of one permutation."""
+    from sage_b200 import _lib
+    from sage_b200.experts import SAGEExperts, expert_slice, synthetic_expert_stack
+
+    assert _lib.load().sageb200_expert_mlp_fits(rows, hidden, inter, 64) == 1
+    assert _lib.load().sageb200_expert_mlp_fits(16, 3456, 128, 64) == 0
+    experts = 33
+    stacks = [synthetic_expert_stack(k, n, experts, 31 + j, "cuda", direction_bits=6)
+              for j, (k, n) in enumerate(((hidden, inter), (hidden, inter), (inter, hidden)))]
+    module = SAGEExperts(*stacks)
+    x = torch.randn(experts, rows, hidden, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").half()
+    got = module.forward_blocks(x, torch.arange(experts, dtype=torch.int32, device="cuda")).float()
+    names = ("packed_codes", "radius_codes", "radius_grid", "codebook", "permutation")
+    for b in (0, experts - 1):
+        gate, up, down = (sage_dequantize(*[expert_slice(stack, b)[key] for key in names], n).float()
+                          for stack, n in zip(stacks, (inter, inter, hidden)))
+        want = (torch.nn.functional.silu(x[b].float() @ gate.T) * (x[b].float() @ up.T)).half().float() @ down.T
+        assert ((got[b] - want).norm(dim=-1) / want.norm(dim=-1)).max() < 2e-3
+
+
 @pytest.mark.parametrize("rows", [512, 515, 1026])
 @pytest.mark.parametrize("hidden", [128, 2560])
 def test_permuting_passes_of_four_rows(rows, hidden):
