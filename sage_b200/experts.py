@@ -61,7 +61,7 @@ def route(logits: torch.Tensor, top_k: int) -> tuple[torch.Tensor, torch.Tensor]
 
 
 ROWS_PER_EXPERT = 16  # rows one expert takes per step (the decode kernel's row limit)
-GROUPED_BLOCKS = 32   # blocks whose gate and up projections one grouped launch takes
+GROUPED_BLOCKS = 32   # see `SAGEExperts.forward`
 
 
 def _on(device: torch.device):
@@ -268,10 +268,13 @@ class SAGEExperts(nn.Module):
         blocks, count, hidden = rows.shape
         lib = _lib.load()
         stacks = self._stacks()
-        # (gate and up of up to 32 blocks fit one grouped launch of the decode kernel, which shares the SMs out evenly
-        #  between them; more blocks would be a chain of such launches, most of whose problems are empty)
-        if blocks > GROUPED_BLOCKS and stacks is not None and lib.sageb200_expert_mlp_fits(count, self.hidden, self.intermediate,
-                                                               max(stack.entries for stack in stacks)):
+        # A few blocks are better off in grouped launches of the decode kernel, which share the SMs out between them, where
+        # the two launches of the expert kernel give each warp whole weight tiles and leave SMs idle.  Measured, grouped /
+        # two launches (us, all blocks live): hidden 2048, intermediate 768, 8 rows: 8 blocks 37 / 41, 16 45 / 43, 24 57 /
+        # 47, 32 68 / 55; 1024, 256: 16 33 / 27; 2560, 1536: 8 51 / 57, 16 74 / 74, 24 94 / 76.  One row (no staging
+        # launch): 16 blocks 37 / 43, 24 47 / 47, 32 61 / 55.  Both are equally far from 64 bits (7.0e-4 to 8.0e-4).
+        if blocks >= (24 if count == 1 else 16) and stacks is not None and lib.sageb200_expert_mlp_fits(
+                count, self.hidden, self.intermediate, max(stack.entries for stack in stacks)):
             # gate, up, SwiGLU and down of all blocks in two launches
             rows = rows.contiguous()
             ids = block_experts if block_experts.dtype == torch.int32 else block_experts.to(torch.int32)

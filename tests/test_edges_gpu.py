@@ -334,3 +334,25 @@ def test_gate_and_up_one_after_another(rows, fused):
         assert torch.equal(both[i], alone)
     if fused:
         assert torch.equal(residuals[0], x + delta)
+
+
+@pytest.mark.parametrize("rows,edge", [(1, 24), (2, 16), (8, 16), (16, 16)])
+def test_expert_blocks_on_both_sides_of_the_rule(rows, edge):
+    """Grouped launches below `edge` blocks, two launches from there: both within FP16 rounding of FP64 on the dense
+    weights (weights, gate, up, activation and result are each rounded once: 5 * 2^-11 / sqrt(3) = 1.4e-3 at most)."""
+    from sage_b200.experts import SAGEExperts, expert_slice, synthetic_expert_stack
+
+    hidden, inter = 512, 384
+    shapes = ((hidden, inter), (hidden, inter), (inter, hidden))
+    stacks = [synthetic_expert_stack(k, n, edge, 51 + j, "cuda") for j, (k, n) in enumerate(shapes)]
+    module = SAGEExperts(*stacks)
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(edge, rows, hidden, generator=gen, device="cuda").half()
+    names = ("packed_codes", "radius_codes", "radius_grid", "codebook", "permutation")
+    for blocks in (edge - 1, edge):
+        got = module.forward_blocks(x[:blocks], torch.arange(blocks, dtype=torch.int32, device="cuda")).double()
+        for b in (0, blocks - 1):
+            gate, up, down = (sage_dequantize(*[expert_slice(stack, b)[key] for key in names], n).double()
+                              for stack, (_, n) in zip(stacks, shapes))
+            want = (torch.nn.functional.silu(x[b].double() @ gate.T) * (x[b].double() @ up.T)) @ down.T
+            assert ((got[b] - want).norm() / want.norm()) < 1.4e-3
