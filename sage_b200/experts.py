@@ -61,7 +61,6 @@ def route(logits: torch.Tensor, top_k: int) -> tuple[torch.Tensor, torch.Tensor]
 
 
 ROWS_PER_EXPERT = 16  # rows one expert takes per step (the decode kernel's row limit)
-GROUPED_BLOCKS = 32   # see `SAGEExperts.forward`
 
 
 def _on(device: torch.device):
@@ -322,11 +321,12 @@ class SAGEExperts(nn.Module):
         parallelism), which saves zero-filling the slot buffers."""
         tokens, top_k = expert_ids.shape
         slots = tokens * top_k
-        if tokens > 1 and GROUPED_BLOCKS < self.experts + (slots + 7) // 8 and self.experts <= 256 and slots <= 4096 \
-                and x.is_cuda and x.dtype == torch.float16:
-            # Several tokens over many experts: slots sorted by expert, each expert's packed bytes decoded once.
-            # Measured for 128 experts, top 8, against one problem per slot: 2 tokens 89 -> 64 us,
-            # 16 tokens 204 -> 119 us (one token: the slots are as many experts already).
+        if tokens > 1 and 32 < slots <= 4096 and self.experts <= 256 and x.is_cuda and x.dtype == torch.float16:
+            # Slots sorted by expert, each expert's packed bytes decoded once; up to 32 slots one problem per slot, whose
+            # launches fill the device as well and need no plan.  Measured at hidden 2048, intermediate 768, slots /
+            # sorted (us, in a captured graph; eager calls cross at the same line): 128 experts, top 8: 16 slots 39 / 57, 32
+            # 61 / 68, 40 78 / 68, 64 107 / 94, 128 193 / 119; 16 experts, top 8: 16 39 / 57, 32 61 / 55, 64 104 / 64; 16 of
+            # 128 experts here: 16 37 / 50, 32 62 / 49, 64 100 / 51.  1024, 256, 32 experts: 32 35 / 37, 64 49 / 37.
             return dispatch_combine(x, expert_ids, weights, self.forward_blocks, first_expert=self.first_expert,
                                     local_experts=self.experts, rows_per_block=8)
         ids = expert_ids.reshape(-1).contiguous()

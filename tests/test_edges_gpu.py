@@ -356,3 +356,39 @@ def test_expert_blocks_on_both_sides_of_the_rule(rows, edge):
                               for stack, (_, n) in zip(stacks, shapes))
             want = (torch.nn.functional.silu(x[b].double() @ gate.T) * (x[b].double() @ up.T)) @ down.T
             assert ((got[b] - want).norm() / want.norm()) < 1.4e-3
+
+
+@pytest.mark.parametrize("experts,first,top_k", [(1, 0, 1), (3, 2, 2), (8, 0, 8), (40, 5, 5)])
+@pytest.mark.parametrize("foreign", [False, True])
+def test_experts_on_both_sides_of_the_slot_rule(experts, first, top_k, foreign):
+    """One problem per slot up to 32 slots, sorted by expert beyond: tokens on both sides, one expert for all of them,
+    experts of other ranks and empty slots (a share of zero), against FP64 on the dense weights."""
+    from sage_b200.experts import SAGEExperts, expert_slice, synthetic_expert_stack
+
+    hidden, inter = 256, 384
+    shapes = ((hidden, inter), (hidden, inter), (inter, hidden))
+    stacks = [synthetic_expert_stack(k, n, experts, 61 + j, "cuda", first=first) for j, (k, n) in enumerate(shapes)]
+    module = SAGEExperts(*stacks, first_expert=first)
+    names = ("packed_codes", "radius_codes", "radius_grid", "codebook", "permutation")
+    dense = [[sage_dequantize(*[expert_slice(stack, e)[key] for key in names], n).double() for e in range(experts)]
+             for stack, (_, n) in zip(stacks, shapes)]
+    for tokens in sorted({2, 32 // top_k, 32 // top_k + 1, 60}):
+        gen = torch.Generator(device="cuda").manual_seed(tokens)
+        x = torch.randn(tokens, hidden, generator=gen, device="cuda").half()
+        ids = torch.stack([torch.randperm(experts, generator=gen, device="cuda")[:top_k] for _ in range(tokens)]) + first
+        ids = ids.to(torch.int32)
+        if foreign:
+            ids[0], ids[1, 0], ids[-1, -1] = first + experts, -1, first - 1
+        weights = torch.rand(tokens, top_k, generator=gen, device="cuda")
+        got = module(x, ids, weights, foreign_experts=foreign).double()
+        want = torch.zeros_like(got)
+        for t in range(tokens):
+            for j in range(top_k):
+                e = int(ids[t, j]) - first
+                if 0 <= e < experts:
+                    act = torch.nn.functional.silu(x[t].double() @ dense[0][e].T) * (x[t].double() @ dense[1][e].T)
+                    want[t] += weights[t, j].double() * (act @ dense[2][e].T)
+        # (rounded once each: weights, gate, up, activation, the slot's result, the mix: 6 * 2^-11 / sqrt(3) at most)
+        assert (got - want).norm() <= 1.7e-3 * want.norm(), tokens
+        if foreign:
+            assert not got[0].any()
