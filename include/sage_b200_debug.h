@@ -44,14 +44,15 @@ int sageb200_set_pdl(int enabled);
 int sageb200_debug_trace(void *device_buffer);
 
 /*
- * The tcgen05 GEMM (rows >= 33) runs as clusters of two CTAs with cta_group::2 MMAs whenever the
+ * The tcgen05 GEMM runs as clusters of two CTAs with cta_group::2 MMAs whenever the
  * shape allows it; 0 switches that off for A/B timing (process-wide, not thread-safe).
  * No counterpart in the reference.
  */
 int sageb200_debug_gemm_pairs(int enabled);
 
 /*
- * The tile plan the tcgen05 GEMM would use for a shape (host arithmetic, no GPU needed), rows >= 33:
+ * The tile plan of the tcgen05 GEMM for a call that takes it - above 32 rows every one, from 9 rows those of large
+ * matrices; the others are refused - as host arithmetic, no GPU needed:
  * fields[0] tokens per accumulator, [1] token blocks, [2] blocks of 128 output rows, [3]
  * accumulators per CTA, [4] CTA pairs (cta_group::2), [5] K splits, [6] 128-channel groups per
  * split, [7] pipeline stages, [8] dynamic shared memory bytes, [9] FP32 scratch of the split tiles in

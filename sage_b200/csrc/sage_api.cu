@@ -1071,7 +1071,8 @@ int sageb200_clear_status(void) {
 }
 
 int sageb200_debug_gemm_plan(int rows, int n, int k, int sm_count, int allow_split, int *fields) {
-  if (!fields || rows < 33 || rows > 65535 || n <= 0 || k <= 0 || (k % 128)) return SAGEB200_ERR_INVALID_ARGUMENT;
+  if (!fields || rows < 1 || rows > 65535 || n <= 0 || k <= 0 || (k % 128) || !takes_gemm(rows, n, k))
+    return SAGEB200_ERR_INVALID_ARGUMENT;
   const GemmPlan plan = plan_gemm_tc(rows, n, k, sm_count > 0 ? sm_count : 148, allow_split != 0);
   fields[0] = plan.tokens_per_cta;
   fields[1] = plan.token_blocks;

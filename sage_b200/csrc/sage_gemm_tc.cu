@@ -113,7 +113,7 @@ __device__ __forceinline__ uint32_t exact_pair(uint32_t direction, float radius)
 // ---------------------------------------------------------------- the kernel
 
 // Dynamic shared memory, 1024-byte aligned by hand:
-//   [A stages: stages x 16 KiB][B stages: stages x TN*128][codebook 4 KiB][barriers]
+//   [A stages: stages x 16 KiB][B stages: stages x TN*128][codebook 32 KiB][barriers]
 // kPair: the grid is launched in clusters of two CTAs along x (two neighbouring row blocks) that
 // run cta_group::2 MMAs.  Both CTAs decode their own 128 rows and load their own half of every
 // activation tile; the even CTA (the leader) issues the MMAs and owns the "stage full" barriers:

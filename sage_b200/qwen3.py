@@ -623,8 +623,8 @@ class PackedQwen3:
         """Run `prompt` [batch, length] into the cache; after it, `self.tokens` holds the first
         generated token.  `batched` (the default on one GPU for a dense-MLP config): all
         prompt tokens go through each layer together - packed linears on the tensor-core GEMM
-        path from 33 rows up, causal attention over the prompt.  Otherwise the prompt is fed
-        one position at a time through the decode graph."""
+        path from 33 rows up (large matrices from 9), causal attention over the prompt.  Otherwise
+        the prompt is fed one position at a time through the decode graph."""
         if self.graph is None:
             self.capture()
         if prompt.dim() != 2 or prompt.shape[0] != self.batch:

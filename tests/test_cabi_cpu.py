@@ -213,3 +213,12 @@ def test_grouped_scratch_of_a_group_that_runs_as_two_launches():
     assert need(even) > max(need(even[:3]), need(even[3:]))
     assert need(even) == need(even) and need(mixed) % 256 == 0
     assert need([(17, 4096, 2560)]) == 0  # more than 16 rows: not a grouped problem
+
+
+def test_gemm_plans_of_few_rows(lib):
+    """The shapes of 9..32 rows that take the GEMM have a plan to show, the decode kernel's are refused."""
+    for rows, n, k in [(24, 2560, 9728), (17, 1024, 2560), (16, 2560, 9728), (9, 25600, 5120), (11, 12288, 4096)]:
+        plan = _gemm_plan(lib, rows, n, k)
+        assert plan["tokens"] * plan["token_blocks"] >= rows and plan["row_blocks"] == (n + 127) // 128
+    for rows, n, k in [(0, 2560, 9728), (8, 25600, 5120), (16, 9728, 2560), (12, 2560, 9728), (24, 512, 2560)]:
+        assert lib.sageb200_debug_gemm_plan(rows, n, k, 148, 1, (ctypes.c_int * 10)()) == -1
