@@ -16,7 +16,8 @@
 //   * two CTAs per SM hide each other's staging.
 // Gate and up of a tile run one after the other in the same warp (their permutations and codebooks differ), so
 // SwiGLU is applied to the accumulators and neither product is stored.
-// Measured, 32 tokens x 8 of 128 experts, hidden 2048, intermediate 768: 300 -> 125 us for the whole exchange.
+// Measured, 32 tokens x 8 of 128 experts, hidden 2048, intermediate 768, the whole exchange:
+// 300 -> 150 us, 97 + 47 of them (under the profiler) in the two launches, whose instructions alone need 66.
 #include "../../include/sage_b200.h"
 #include "sage_common.cuh"
 #include "sage_kernels.h"

@@ -868,6 +868,8 @@ GemmPlan plan_gemm_group(int rows, const int *n, int count, int k, int sm_count,
         if (splits > 1) {
           const double tile_bytes = accumulators * candidate * 128.0 * 4.0;
           cost += 2.0 * per_split * stage + around + 2000.0;
+          // (Two prices for one reduction code, each fitted to the grids that it prices; neither has been measured on the
+          //  other's.  One for all would give 2560 -> 1024 at 77 to 512 rows, 9728 -> 2560 at 300 and others another plan.)
           if (rest_only)  // as below, but by the last CTAs of its three parts; and all of it through L2 (~28 bytes per cycle and SM)
             cost += (1.0 + splits / (splits < 3 ? splits : 3.0)) * tile_bytes / 64.0 +
                     2.0 * (tiles - main) * splits * tile_bytes / (28.0 * sm_count);
